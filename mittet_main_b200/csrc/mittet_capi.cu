@@ -880,12 +880,16 @@ int launch_persistent(mittet_handle *h, int vi, int grid, const PersistArgs<T> &
     return MITTET_OK;
 }
 
-// Device time of one replay of a graph (after one untimed replay).
+// Device time of one replay of a graph (after one untimed replay).  The
+// captured steps write traces and read the wavelet at the device's step
+// counter, so every replay starts from step 0.
 int time_graph(mittet_handle *h, cudaGraphExec_t g, float *ms) {
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
+    CK(cudaMemsetAsync(h->d_step.p, 0, sizeof(int), h->st));
     CK(cudaGraphLaunch(g, h->st));
+    CK(cudaMemsetAsync(h->d_step.p, 0, sizeof(int), h->st));
     CK(cudaEventRecord(e0, h->st));
     CK(cudaGraphLaunch(g, h->st));
     CK(cudaEventRecord(e1, h->st));
@@ -898,9 +902,10 @@ int time_graph(mittet_handle *h, cudaGraphExec_t g, float *ms) {
 
 // Chooses between the stepped graph of part kernels and the persistent
 // launch for this grid and batch by timing one captured block of G steps of
-// each (MITTET_PERSIST=0 / 1 forces one).  Leaves zero fields behind.
+// each, or of all nt steps where they are fewer: the traces and the wavelet
+// end there (MITTET_PERSIST=0 / 1 forces one).  Leaves zero fields behind.
 std::mutex g_persist_mu;
-std::map<std::array<long long, 8>, int> g_persist_cache;  // choice per (grid, shots, precision, points, ring)
+std::map<std::array<long long, 9>, int> g_persist_cache;  // choice per (grid, shots, precision, points, ring, block)
 
 template <typename T>
 int decide_persistent(mittet_handle *h, const PhaseArgs<T> &ea, const PhaseArgs<T> &ha, const InjectArgs<T> &ia_m,
@@ -911,8 +916,9 @@ int decide_persistent(mittet_handle *h, const PhaseArgs<T> &ea, const PhaseArgs<
     const int force = mode ? std::atoi(mode) : -1;
     if (force == 0) return MITTET_OK;
     CK(h->bar.ensure(sizeof(GridBarrier)));
-    const std::array<long long, 8> key = {h->g.nx, h->g.ny, h->g.nz, h->nshot, (long long)h->fp64 + 2 * (force == 1),
-                                          (long long)h->has_mag + 2 * h->has_ele, ea.ring_k, h->nrec};
+    G = std::min(G, sa.nt);
+    const std::array<long long, 9> key = {h->g.nx, h->g.ny, h->g.nz, h->nshot, (long long)h->fp64 + 2 * (force == 1),
+                                          (long long)h->has_mag + 2 * h->has_ele, ea.ring_k, h->nrec, G};
     if (!std::getenv("MITTET_PERSIST_STALL")) {
         std::lock_guard<std::mutex> lk(g_persist_mu);
         auto it = g_persist_cache.find(key);
