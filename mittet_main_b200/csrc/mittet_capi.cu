@@ -1585,13 +1585,15 @@ int run_forward(mittet_handle *h, int nt) {
         rc = resident_args<T>(h, plan, ns, ea, ha, h->d_pts.as<SrcPoint>(), h->npts, h->traces.as<T>(), nt, &ra);
         if (rc) return rc;
         h->launches = 0;
-        const int per = vol ? h->ring_k : kResidentSteps;
+        const int per = vol ? h->ring_k : nt;  // steps between flushes of the ring
         for (int done = 0; done < nt; done += per) {
-            ra.n0 = done;
-            ra.nsteps = std::min(per, nt - done);
-            CK(resident_launch<T>(ra, plan, h->st));
-            h->launches++;
-            if (vol) launch_volume_flush<T>(h, ra.nsteps, done);
+            const int end = std::min(done + per, nt);
+            for (ra.n0 = done; ra.n0 < end; ra.n0 += ra.nsteps) {
+                ra.nsteps = std::min(plan.steps, end - ra.n0);
+                CK(resident_launch<T>(ra, plan, h->st));
+                h->launches++;
+            }
+            if (vol) launch_volume_flush<T>(h, end - done, done);
         }
         h->resident_ctas = plan.groups * plan.ty * plan.tz;
         return finish_forward<T>(h, nt);
@@ -2143,7 +2145,7 @@ int run_gradient(mittet_handle *h, int nt, const double *obs_host, int K, double
                 rh.hist_comp = (long long)gF;
                 for (int n = n0; n < n1; n += rh.nsteps) {
                     rh.n0 = n;
-                    rh.nsteps = std::min(kResidentSteps, n1 - n);
+                    rh.nsteps = std::min(plan.steps, n1 - n);
                     rh.hist = hist.as<T>() + (size_t)(n - n0) * slot;
                     CK(resident_launch<T>(rh, plan, h->st));
                 }
@@ -2198,7 +2200,7 @@ int run_gradient(mittet_handle *h, int nt, const double *obs_host, int K, double
                 continue;
             }
             ra.n0 = n;
-            ra.nsteps = std::min(kResidentSteps, K - n % K);
+            ra.nsteps = std::min(plan.steps, K - n % K);
             CK(resident_launch<T>(ra, plan, h->st));
             n += ra.nsteps - 1;
         }

@@ -87,6 +87,7 @@ ResPlan resident_plan(int nx, int ny, int nz, const unsigned char *heavy_y, cons
                 best = p;
             }
         }
+    best.steps = best.ok ? std::min(kResidentSteps, std::max(1, (int)(kResidentLaunchUs / (2.0 * best_t)))) : 0;
     return best;
 }
 

@@ -64,10 +64,12 @@ template <>
 struct ResShape<double> {
     static constexpr int VX = 2, NT = 256;
 };
-// Steps of one resident launch without a ring: long enough that loading and
-// storing the tiles does not show, short enough that a launch stays well
-// below a second for a batch.
+// Steps of one resident launch: long enough that loading and storing the
+// tiles does not show, and by the tiling's own estimate no more than half a
+// second for all shots, since nothing else of the process gets the SMs
+// meanwhile (64 shots of 101^3 take 2 ms a step).
 constexpr int kResidentSteps = 1024;
+constexpr double kResidentLaunchUs = 5e5;
 constexpr int kResMaxPts = 32;    // points of one shot
 constexpr int kResRecCache = 128; // receivers of a tile listed in shared memory
 constexpr int kResFlagStride = 32;  // words between flags: one line each
@@ -910,6 +912,7 @@ struct ResPlan {
     int nrow = 0, ry = 0, rz = 0, pitch = 0;  // rows of the largest tile; most rows along y, z; elements per row
     unsigned short ys[kResMaxTiles + 1], zs[kResMaxTiles + 1];
     size_t smem = 0;                          // bytes
+    int steps = 0;                            // most steps of one launch
 };
 
 // The tiling for nshot shots on nsm SMs (resident.cu); heavy_y, heavy_z: rows
