@@ -1022,12 +1022,13 @@ int decide_persistent(mittet_handle *h, const PhaseArgs<T> &ea, const PhaseArgs<
 
 // -------------------------------------------------------- resident launch
 // Whether nshot shots with these points run on the resident launch, and its
-// tiling.  It takes every solve whose fields fit the GPU's shared memory,
-// since it was the faster path on each that was measured (microseconds per
-// step, stepped -> resident): 16^3 24 -> 10, 64^3 25 -> 10.4, 96^3 47 -> 23,
-// 101^3 45 -> 31, 120x80x100 49 -> 33, 33x290x24 35 -> 12, 3 shots of
-// 160x60x90 108 -> 80, 32 shots of 32^3 54 -> 30, of 64^3 321 -> 229; FP64
-// 72^3 45 -> 28, 4 shots of 64^3 104 -> 62.  Points must lie on the field
+// tiling.  It takes every gradient's forward passes and every FP32 solve whose
+// fields fit the GPU's shared memory, since it was the faster path on each that
+// was measured (microseconds per step, stepped -> resident): 16^3 24 -> 10, 64^3
+// 25 -> 10.4, 96^3 45 -> 23, 101^3 46 -> 31, 33x290x24 35 -> 12, 3 shots of
+// 160x60x90 97 -> 77, 16 437 -> 409, 32 shots of 48^3 170 -> 101, of 64^3 329
+// -> 227, of 96^3 936 -> 728, of 101^3 1045 -> 972; and the FP64 solves that
+// fp64_batch_stepped leaves it.  Points must lie on the field
 // their kind drives (magnetic on H, electric on E), where the tile that owns
 // the cell applies them; a shot of more points than a tile lists runs on the
 // stepped path.  The variables that force a stepped or persistent body switch
@@ -1077,6 +1078,33 @@ bool resident_for(mittet_handle *h, int nshot, const mittet_point_source *pts, s
     h->res_plan = *plan;
     h->res_plan_shots = nshot;
     return plan->ok;
+}
+
+// FP64 solves that the stepped path runs faster although they fit: the resident
+// launch computes floor(SMs / tiles) shots at a time, so its time grows with
+// their number, while a stepped launch holds all shots and its cost per cell
+// falls until HBM bounds it.  Microseconds per step, resident and stepped: 64^3
+// x 64 shots 978, 1079; 72^3 x 8 225, 238; x 16 441, 440; x 32 886, 838; with a
+// 16-cell CPML 924, 1029; 80^3 x 4 138, 163; x 8 277, 275; x 32 1105, 1030; x
+// 64 2210, 1957; 84^3 x 8 290, 316; 50x100x80 x 24 685, 713; 120x60x60 x 24
+// 649, 616.  Both estimates are fits to 46 such pairs: a resident phase takes
+// 1 us and 1.95 for each pass of the largest tile (within 9 %); a stepped step
+// 43 us and per cell 0.0107 ns, 0.053 for cells of the CPML, 0.057 times the
+// share of its x faces (32-cell boxes) and 0.017 times the rows' padding (within
+// 7 % from 1.5 M cells on; below that it is too long, in favour of the resident
+// launch).  The stepped path, which tunes itself on a new batch, must be a
+// tenth shorter by them; of the pairs the rule then misses by more than 1 % only
+// 120x60x60 x 24.  MITTET_RESIDENT=1 keeps the resident launch.
+template <typename T>
+bool fp64_batch_stepped(const mittet_handle *h, int nshot, const ResPlan &p) {
+    if (sizeof(T) == 4 || std::getenv("MITTET_RESIDENT")) return false;
+    constexpr int VX = ResShape<T>::VX, NT = ResShape<T>::NT;
+    const double nx = h->g.nx, ny = h->g.ny, nz = h->g.nz, nc = h->g.ncpml;
+    const int rounds = (nshot + p.groups - 1) / p.groups, items = p.ry * p.rz * ((h->g.nx + VX - 1) / VX);
+    const double resident = 2.0 * rounds * (1.0 + 1.95 * ((items + NT - 1) / NT));
+    const double cpml = 1.0 - (nx - 2 * nc) * (ny - 2 * nc) * (nz - 2 * nc) / (nx * ny * nz);
+    const double per_cell = 0.0107 + 0.0532 * cpml + 0.057 * 2.0 * nc / nx + 0.0168 * (h->px / nx - 1.0);
+    return 43.5 + 1e-3 * nshot * nx * ny * nz * per_cell < 0.9 * resident;
 }
 
 // The launch arguments that stay the same over a solve; builds the receiver
@@ -1580,7 +1608,7 @@ int run_forward(mittet_handle *h, int nt) {
 
     ResPlan plan;
     h->resident_ctas = 0;
-    if (resident_for<T>(h, ns, h->pts.data(), h->pts.size(), &plan)) {
+    if (resident_for<T>(h, ns, h->pts.data(), h->pts.size(), &plan) && !fp64_batch_stepped<T>(h, ns, plan)) {
         ResArgs<T> ra;
         rc = resident_args<T>(h, plan, ns, ea, ha, h->d_pts.as<SrcPoint>(), h->npts, h->traces.as<T>(), nt, &ra);
         if (rc) return rc;
