@@ -178,7 +178,7 @@ def serving(args):
         lat = [r.latency for r in res]
         errors = [r.error for r in res if r.error]
         out[name] = {"policy": policy, "p50_s": percentile(lat, 50), "p99_s": percentile(lat, 99), "wall_s": wall,
-                     "shot_solves_per_s": shots / wall, "max_concurrent": srv.max_concurrent,
+                     "shot_solves_per_s": shots / wall, "max_running": srv.max_running,
                      "peak_budget_bytes": srv.peak_in_use, "handle_reuses": srv.reuses,
                      "evictions": srv.evictions, "errors": errors[:3]}
     out["server_vs_one_shot"] = out["server"]["shot_solves_per_s"] / out["one_shot_at_a_time"]["shot_solves_per_s"]
