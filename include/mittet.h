@@ -332,7 +332,10 @@ int64_t mittet_last_launch_count(mittet_handle *h);
  *                positive and finite: unlike mittet_set_model this call does
  *                not read the model back to check it, and it runs no
  *                finite check on the result (a bad model or an unstable dt
- *                gives Inf/NaN spectra, not MITTET_ERR_DIVERGED)
+ *                gives Inf/NaN spectra, not MITTET_ERR_DIVERGED).  All
+ *                spectra are NaN when a bounded wait between the SMs gave up
+ *                (2 s without progress): the call has returned by then, so
+ *                it cannot report MITTET_ERR_DEVICE_TIMEOUT
  *   wavelet_dev: device, nt+1 doubles, w[n] = s(n dt)
  *   pts, rec, omega: host arrays (copied into the device array)
  *   rec_fd_dev:  device output, [nrec][nf] complex (interleaved doubles)

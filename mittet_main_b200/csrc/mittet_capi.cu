@@ -1167,12 +1167,7 @@ int resident_args(mittet_handle *h, const ResPlan &p, int nshot, const PhaseArgs
     a.nt = nt;
     a.flags = h->res_flags.as<unsigned>();
     a.err = h->d_flag.as<int>();
-    // MITTET_RESIDENT_STALL=1 makes every wait ask for a phase that nobody
-    // finishes, so that a test can watch the waits give up
-    const char *stall = std::getenv("MITTET_RESIDENT_STALL");
-    a.expect_more = (stall && std::atoi(stall) == 1) ? 1u << 30 : 0u;
-    const char *wms = std::getenv("MITTET_PERSIST_WAIT_MS");
-    a.wait_ns = (unsigned long long)((wms ? std::max(1.0, std::atof(wms)) : 2000.0) * 1e6);
+    resident_waits(&a);
     return MITTET_OK;
 }
 

@@ -449,7 +449,7 @@ extern "C" int mittet_forward_noalloc(const mittet_grid *g, const mittet_phys *p
         ra.nt = nt;
         ra.flags = (unsigned *)(base + o_flags);
         ra.err = (int *)(base + o_err);
-        ra.wait_ns = 2000000000ull;
+        resident_waits(&ra);
         for (ra.n0 = 0; ra.n0 < nt; ra.n0 += ra.nsteps) {
             ra.nsteps = std::min(plan.steps, nt - ra.n0);
             NA_CK(resident_launch<float>(ra, plan, st));

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -92,6 +93,13 @@ ResPlan resident_plan(int nx, int ny, int nz, const unsigned char *heavy_y, cons
 }
 
 template <typename T>
+void resident_waits(ResArgs<T> *a) {
+    const char *stall = std::getenv("MITTET_RESIDENT_STALL"), *wms = std::getenv("MITTET_PERSIST_WAIT_MS");
+    a->expect_more = (stall && std::atoi(stall) == 1) ? 1u << 30 : 0u;
+    a->wait_ns = (unsigned long long)((wms ? std::max(1.0, std::atof(wms)) : 2000.0) * 1e6);
+}
+
+template <typename T>
 cudaError_t resident_launch(const ResArgs<T> &a, const ResPlan &p, cudaStream_t st) {
     // an attribute of the current device's function: set for each launch
     cudaError_t e = cudaFuncSetAttribute(resident_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 1024);
@@ -115,6 +123,8 @@ cudaError_t resident_launch(const ResArgs<T> &a, const ResPlan &p, cudaStream_t 
 
 template ResPlan resident_plan<float>(int, int, int, const unsigned char *, const unsigned char *, int, int);
 template ResPlan resident_plan<double>(int, int, int, const unsigned char *, const unsigned char *, int, int);
+template void resident_waits<float>(ResArgs<float> *);
+template void resident_waits<double>(ResArgs<double> *);
 template cudaError_t resident_launch<float>(const ResArgs<float> &, const ResPlan &, cudaStream_t);
 template cudaError_t resident_launch<double>(const ResArgs<double> &, const ResPlan &, cudaStream_t);
 

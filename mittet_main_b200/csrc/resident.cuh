@@ -921,6 +921,12 @@ template <typename T>
 ResPlan resident_plan(int nx, int ny, int nz, const unsigned char *heavy_y, const unsigned char *heavy_z, int nshot,
                       int nsm);
 
+// Limits of the launch's waits (resident.cu): MITTET_PERSIST_WAIT_MS, and with
+// MITTET_RESIDENT_STALL=1 every wait asks for a phase that nobody finishes, so
+// that a test can watch the waits give up.
+template <typename T>
+void resident_waits(ResArgs<T> *a);
+
 // One cooperative launch of a.nsteps steps (resident.cu).
 template <typename T>
 cudaError_t resident_launch(const ResArgs<T> &a, const ResPlan &p, cudaStream_t st);
