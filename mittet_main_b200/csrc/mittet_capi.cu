@@ -467,6 +467,15 @@ TileMap make_tilemap(const mittet_handle *h, bool e, int vx, int bx, int by, int
     return t;
 }
 
+// Host data to a buffer of the handle, behind the work queued on its stream: a
+// solve in flight (mittet_forward_device returns before it) keeps what it was
+// started with, and the next one reads the new data.  The bytes have left src
+// when the call returns (pageable memory is staged).
+int put(mittet_handle *h, void *dst, const void *src, size_t bytes) {
+    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->st));
+    return MITTET_OK;
+}
+
 template <typename T>
 int upload_tilemaps(mittet_handle *h) {
     const auto &vs = variants<T>();
@@ -491,9 +500,8 @@ int upload_tilemaps(mittet_handle *h) {
     }
     h->tmaps_host = maps;
     CK(h->tmaps.ensure(maps.size() * sizeof(TileMap)));
-    CK(cudaMemcpy(h->tmaps.p, maps.data(), maps.size() * sizeof(TileMap), cudaMemcpyHostToDevice));
     drop_graph(h);
-    return MITTET_OK;
+    return put(h, h->tmaps.p, maps.data(), maps.size() * sizeof(TileMap));
 }
 
 // ------------------------------------------------- TMA-staged interior
@@ -2545,11 +2553,11 @@ int mittet_create(const mittet_grid *g, const mittet_phys *ph, mittet_handle **o
     cudaError_t e = h->prof.ensure(np * h->esz);
     if (e == cudaSuccess) {
         if (h->fp64) {
-            e = cudaMemcpy(h->prof.p, h->su.prof.data(), np * 8, cudaMemcpyHostToDevice);
+            e = cudaMemcpyAsync(h->prof.p, h->su.prof.data(), np * 8, cudaMemcpyHostToDevice, h->st);
         } else {
             std::vector<float> pf(np);
             for (size_t q = 0; q < np; q++) pf[q] = (float)h->su.prof[q];
-            e = cudaMemcpy(h->prof.p, pf.data(), np * 4, cudaMemcpyHostToDevice);
+            e = cudaMemcpyAsync(h->prof.p, pf.data(), np * 4, cudaMemcpyHostToDevice, h->st);
         }
     }
     if (e != cudaSuccess) {
@@ -2721,7 +2729,7 @@ int mittet_set_wavelet(mittet_handle *h, int32_t nt, const double *w) {
     int rc = set_device(h);
     if (rc) return rc;
     CK(h->wave.ensure((size_t)(nt + 1) * 8));
-    CK(cudaMemcpy(h->wave.p, w, (size_t)(nt + 1) * 8, cudaMemcpyHostToDevice));
+    if ((rc = put(h, h->wave.p, w, (size_t)(nt + 1) * 8))) return rc;
     h->nt_wave = nt;
     drop_graph(h);
     return MITTET_OK;
@@ -2747,9 +2755,9 @@ int mittet_set_receivers(mittet_handle *h, int32_t nrec, const mittet_receiver *
     CK(h->rec_off.ensure(off.size() * 8));
     CK(h->rec_comp.ensure(comp.size() * 4));
     CK(h->rec_is_h.ensure(ish.size()));
-    CK(cudaMemcpy(h->rec_off.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->rec_comp.p, comp.data(), comp.size() * 4, cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(h->rec_is_h.p, ish.data(), ish.size(), cudaMemcpyHostToDevice));
+    if ((rc = put(h, h->rec_off.p, off.data(), off.size() * 8)) || (rc = put(h, h->rec_comp.p, comp.data(), comp.size() * 4)) ||
+        (rc = put(h, h->rec_is_h.p, ish.data(), ish.size())))
+        return rc;
     h->nrec = nrec;
     h->recs.assign(rec, rec + nrec);
     h->res_ty = h->res_tz = 0;
@@ -2766,7 +2774,7 @@ int mittet_set_freqs(mittet_handle *h, int32_t nf, const double *omega, int32_t 
     h->omega.assign(omega, omega + nf);
     h->hfac = h_factor ? 1 : 0;
     CK(h->d_omega.ensure(std::max(nf, 1) * 8));
-    if (nf) CK(cudaMemcpy(h->d_omega.p, omega, nf * 8, cudaMemcpyHostToDevice));
+    if (nf && (rc = put(h, h->d_omega.p, omega, nf * 8))) return rc;
     drop_graph(h);
     return MITTET_OK;
 }
@@ -2864,6 +2872,7 @@ int mittet_get_fields(mittet_handle *h, int32_t shot, double *out) {
     int rc = set_device(h);
     if (rc) return rc;
     const size_t n = (size_t)h->g.nx * h->g.ny * h->g.nz;
+    CK(cudaStreamSynchronize(h->st));
     for (int c = 0; c < 6; c++) {
         const char *base = (const char *)h->fields[c].p + (size_t)shot * h->fshot * h->esz;
         if (h->fp64) {

@@ -1,0 +1,45 @@
+"""GPU: work queued on other streams than the handle's own, and calls made while
+a solve that returned early (forward_device) still runs."""
+from dataclasses import replace
+
+import numpy as np
+import pytest
+
+from mittet_main_b200 import workloads as W
+from mittet_main_b200.capi import FP32
+
+pytestmark = pytest.mark.gpu
+
+
+def case(nt=1500):
+    return W.small_case(n=(40, 36, 32), ncpml=8, nt=nt, precision=FP32, seed=6)
+
+
+@pytest.mark.parametrize("resident", [True, False])
+def test_a_solve_in_flight_keeps_what_it_was_started_with(monkeypatch, resident):
+    """The wavelet, receivers, frequencies and shots of the next solve are set
+    while the last one runs; its spectra and fields are its own."""
+    import torch
+
+    if not resident:
+        monkeypatch.setenv("MITTET_RESIDENT", "0")
+    wl = case()
+    out = torch.zeros((1, len(wl.receivers), len(wl.omega), 2), dtype=torch.float64, device="cuda")
+    with W.make_solver(wl) as s:
+        want, _ = s.forward(wl.nt)
+        want_f = s.fields(0)
+        assert np.abs(want).max() > 0
+        for change in (lambda: s.set_wavelet(0.5 * wl.wavelet), lambda: s.set_receivers(wl.receivers[::-1]),
+                       lambda: s.set_freqs(2.0 * wl.omega), lambda: s.set_shots([wl.shots[0]] * 2)):
+            torch.cuda.synchronize()
+            s.forward_device(wl.nt, out, torch.cuda.current_stream())
+            change()
+            torch.cuda.synchronize()
+            got = out.cpu().numpy()
+            assert np.array_equal(got[..., 0] + 1j * got[..., 1], want)
+            s.set_wavelet(wl.wavelet)
+            s.set_receivers(wl.receivers)
+            s.set_freqs(wl.omega)
+            s.set_shots(wl.shots)
+        s.forward_device(wl.nt, out, torch.cuda.current_stream())
+        assert np.array_equal(s.fields(0), want_f)  # read behind the solve
