@@ -240,7 +240,9 @@ int mittet_satan_gamma(int32_t device, const mittet_grid *grid, int32_t nrec, co
  * stream is the caller's cudaStream_t (NULL = the legacy default stream): the
  * solve starts after the work already queued there and the stream waits for
  * the solve, so events recorded on it bracket the whole solve.
- * mittet_set_model_device: sigma (and mu, or NULL) are [nz][ny][nx] arrays of
+ * mittet_set_model_device reads its arrays after the work queued on the
+ * legacy default stream; one written on another stream must be complete.  It
+ * has read them when it returns.  sigma (and mu, or NULL) are [nz][ny][nx] arrays of
  * double (is_fp64 = 1) or float (0), whatever the handle's precision; the
  * model stays on the device (checked there: MITTET_ERR_INVALID_ARG for a
  * value that is not positive and finite), and m = 2 w0 dt / sigma is formed

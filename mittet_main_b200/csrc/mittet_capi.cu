@@ -2639,6 +2639,16 @@ int mittet_set_model(mittet_handle *h, const double *sigma, const double *mu) {
     return upload_sources(h);
 }
 
+// The handle's stream continues after the work queued on a caller's stream.
+static int wait_for(mittet_handle *h, cudaStream_t user) {
+    cudaEvent_t ev;
+    CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    CK(cudaEventRecord(ev, user));
+    CK(cudaStreamWaitEvent(h->st, ev, 0));
+    cudaEventDestroy(ev);
+    return MITTET_OK;
+}
+
 int mittet_set_model_device(mittet_handle *h, const void *sigma, const void *mu, int32_t is_fp64) {
     if (!h || !sigma) return fail(MITTET_ERR_INVALID_ARG, "null argument");
     int rc = set_device(h);
@@ -2647,6 +2657,7 @@ int mittet_set_model_device(mittet_handle *h, const void *sigma, const void *mu,
     // the model stays on the device: a device-side check (a rejected model
     // leaves the handle's model as it was), then an FP64 stage that the
     // source gains read their few cells from; no host round trip
+    if ((rc = wait_for(h, cudaStreamLegacy))) return rc;
     CK(h->d_flag.ensure(sizeof(int)));
     CK(cudaMemsetAsync(h->d_flag.p, 0, sizeof(int), h->st));
     auto stage = [&](double *s64, double *m64) {
@@ -2828,13 +2839,7 @@ int mittet_forward_device(mittet_handle *h, int32_t nt, void *rec_fd_dev, void *
     // the caller's stream; NULL is the legacy default stream, which the
     // handle's non-blocking stream does not synchronise with implicitly
     cudaStream_t user = stream ? (cudaStream_t)stream : cudaStreamLegacy;
-    {
-        cudaEvent_t ev;
-        CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        CK(cudaEventRecord(ev, user));
-        CK(cudaStreamWaitEvent(h->st, ev, 0));
-        cudaEventDestroy(ev);
-    }
+    if ((rc = wait_for(h, user))) return rc;
     rc = h->fp64 ? run_forward<double>(h, nt) : run_forward<float>(h, nt);
     if (rc) return rc;
     const int nf = (int)h->omega.size();

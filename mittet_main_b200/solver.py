@@ -164,7 +164,8 @@ class MittetSolver:
     def set_model_device(self, sigma, mu=None):
         """sigma/mu as contiguous [nz, ny, nx] CUDA torch tensors (float64 or
         float32, both the same) on the handle's device; the model stays on the
-        device."""
+        device.  Waits for the work queued on torch's current stream, which
+        may still be writing them."""
         import torch
 
         if sigma.dtype not in (torch.float64, torch.float32) or not sigma.is_cuda or not sigma.is_contiguous():
@@ -174,6 +175,7 @@ class MittetSolver:
         if mu is not None and (mu.dtype != sigma.dtype or mu.shape != sigma.shape or not mu.is_cuda
                                or not mu.is_contiguous()):
             raise ValueError("mu must be a contiguous CUDA tensor of sigma's dtype and shape")
+        torch.cuda.current_stream(sigma.device).synchronize()
         check(self._lib.mittet_set_model_device(self._h, ctypes.c_void_p(sigma.data_ptr()),
                                                 ctypes.c_void_p(mu.data_ptr()) if mu is not None else None,
                                                 1 if sigma.dtype == torch.float64 else 0))

@@ -43,3 +43,23 @@ def test_a_solve_in_flight_keeps_what_it_was_started_with(monkeypatch, resident)
             s.set_shots(wl.shots)
         s.forward_device(wl.nt, out, torch.cuda.current_stream())
         assert np.array_equal(s.fields(0), want_f)  # read behind the solve
+
+
+@pytest.mark.parametrize("own_stream", [False, True])
+def test_a_device_model_is_read_after_the_work_that_writes_it(own_stream):
+    import torch
+
+    wl = case(nt=60)
+    sig = torch.from_numpy(np.ascontiguousarray(wl.sigma)).cuda()
+    late = torch.full_like(sig, 0.7)
+    busy = torch.empty(1 << 28, dtype=torch.float32, device="cuda")
+    with W.make_solver(wl) as s:
+        want, _ = s.forward(wl.nt)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(torch.cuda.Stream() if own_stream else torch.cuda.current_stream()):
+            for _ in range(60):  # about 20 ms of writes before the model's
+                busy.fill_(1.0)
+            late.copy_(sig)
+            s.set_model_device(late)
+        got, _ = s.forward(wl.nt)
+    assert np.array_equal(got, want)
