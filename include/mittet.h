@@ -248,6 +248,11 @@ int mittet_satan_gamma(int32_t device, const mittet_grid *grid, int32_t nrec, co
  * value that is not positive and finite), and m = 2 w0 dt / sigma is formed
  * in FP64 from the given values as mittet_set_model does. */
 int mittet_set_model_device(mittet_handle *h, const void *sigma, const void *mu, int32_t is_fp64);
+/* mittet_forward_device: rec_fd_dev (or NULL) receives [nshot][nrec][nf]
+ * complex, as mittet_forward's rec_fd.  The call returns before the solve
+ * ends, so a solve that diverged or in which a bounded wait gave up is not
+ * reported by its return code: the first leaves Inf/NaN in the spectra it
+ * reaches, the second NaN in all of them. */
 int mittet_forward_device(mittet_handle *h, int32_t nt, void *rec_fd_dev, void *stream);
 
 /* Per-kernel timing of the stepped path (CUDA events on the handle's stream):

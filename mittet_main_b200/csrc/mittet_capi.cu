@@ -2639,6 +2639,13 @@ int mittet_set_model(mittet_handle *h, const double *sigma, const double *mu) {
     return upload_sources(h);
 }
 
+// A wait inside the time loop that gave up leaves no result: NaN in its place.
+static __global__ void stalled_kernel(const int *__restrict__ err, double *__restrict__ out, long long n) {
+    if (!(*err & 6)) return;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+        out[e] = nan("");
+}
+
 // The handle's stream continues after the work queued on a caller's stream.
 static int wait_for(mittet_handle *h, cudaStream_t user) {
     cudaEvent_t ev;
@@ -2844,8 +2851,11 @@ int mittet_forward_device(mittet_handle *h, int32_t nt, void *rec_fd_dev, void *
     if (rc) return rc;
     const int nf = (int)h->omega.size();
     const size_t ntr = (size_t)h->nshot * h->nrec;
-    if (rec_fd_dev && nf > 0 && ntr > 0)
+    if (rec_fd_dev && nf > 0 && ntr > 0) {
         CK(cudaMemcpyAsync(rec_fd_dev, h->spectra.p, ntr * nf * sizeof(double2), cudaMemcpyDeviceToDevice, h->st));
+        stalled_kernel<<<16, 256, 0, h->st>>>(h->d_flag.as<int>(), (double *)rec_fd_dev, (long long)ntr * nf * 2);
+        CK(cudaGetLastError());
+    }
     {
         cudaEvent_t ev;
         CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));

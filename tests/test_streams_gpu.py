@@ -1,5 +1,5 @@
-"""GPU: work queued on other streams than the handle's own, and calls made while
-a solve that returned early (forward_device) still runs."""
+"""GPU: work queued on other streams than the handle's own, calls made while a
+solve that returned early (forward_device) still runs, and its failures."""
 from dataclasses import replace
 
 import numpy as np
@@ -63,3 +63,26 @@ def test_a_device_model_is_read_after_the_work_that_writes_it(own_stream):
             s.set_model_device(late)
         got, _ = s.forward(wl.nt)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("stall,env", [("MITTET_RESIDENT_STALL", {}), ("MITTET_PERSIST_STALL", {"MITTET_PERSIST": "1"})])
+def test_a_stalled_device_solve_leaves_nan(monkeypatch, stall, env):
+    import torch
+
+    wl = case(nt=150)
+    out = torch.full((1, len(wl.receivers), len(wl.omega), 2), 7.0, dtype=torch.float64, device="cuda")
+    with W.make_solver(wl) as s:
+        want, _ = s.forward(wl.nt)
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    monkeypatch.setenv(stall, "1")
+    monkeypatch.setenv("MITTET_PERSIST_WAIT_MS", "20")
+    with W.make_solver(wl) as s:
+        s.forward_device(wl.nt, out, torch.cuda.current_stream())
+        assert torch.isnan(out).all()
+    monkeypatch.delenv(stall)
+    monkeypatch.delenv("MITTET_PERSIST_WAIT_MS")
+    with W.make_solver(wl) as s:
+        s.forward_device(wl.nt, out, torch.cuda.current_stream())
+    got = out.cpu().numpy()
+    assert np.array_equal(got[..., 0] + 1j * got[..., 1], want)
