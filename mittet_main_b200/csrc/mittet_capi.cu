@@ -1545,13 +1545,10 @@ int finish_forward(mittet_handle *h, int nt) {
     return MITTET_OK;
 }
 
-template <typename T>
-int run_forward(mittet_handle *h, int nt) {
+// Buffers and volume weights of a solve of nt steps with the handle's present
+// shots, receivers and frequencies; step counter, flags and volume sums zero.
+int solve_buffers(mittet_handle *h, int nt) {
     const int ns = h->nshot;
-    int rc = ensure_state(h);
-    if (rc) return rc;
-    rc = ensure_part_streams(h);
-    if (rc) return rc;
     CK(h->d_step.ensure(sizeof(int)));
     CK(h->d_flag.ensure(sizeof(int)));
     CK(cudaMemsetAsync(h->d_step.p, 0, sizeof(int), h->st));
@@ -1577,6 +1574,19 @@ int run_forward(mittet_handle *h, int nt) {
                 wt[((size_t)n * nf + f) * 2 + 1] = e * std::sin(xa);
             }
     }
+    return MITTET_OK;
+}
+
+template <typename T>
+int run_forward(mittet_handle *h, int nt) {
+    const int ns = h->nshot;
+    int rc = ensure_state(h);
+    if (rc) return rc;
+    rc = ensure_part_streams(h);
+    if (rc) return rc;
+    if ((rc = solve_buffers(h, nt))) return rc;
+    const int nf = (int)h->omega.size();
+    const bool vol = h->vmask && nf > 0;
 
     PhaseArgs<T> ea = phase_args<T>(h, true);
     PhaseArgs<T> ha = phase_args<T>(h, false);
@@ -1726,6 +1736,7 @@ int time_kernels(mittet_handle *h, int nsteps, double *ms) {
     rc = ensure_part_streams(h);
     if (rc) return rc;
     const int nt = h->last_nt;
+    if ((rc = solve_buffers(h, nt))) return rc;
     const bool vol = h->vmask && !h->omega.empty();
     PhaseArgs<T> ea = phase_args<T>(h, true);
     PhaseArgs<T> ha = phase_args<T>(h, false);
@@ -2873,6 +2884,8 @@ int mittet_get_volume_dft(mittet_handle *h, int32_t shot, int32_t comp, double *
     int rc = set_device(h);
     if (rc) return rc;
     const int nf = (int)h->omega.size();
+    if (((size_t)h->nshot * 3 * nf) * h->fshot * sizeof(double2) > h->acc.bytes)
+        return fail(MITTET_ERR_STATE, "run a forward with these shots and frequencies first");
     const double2 *base = h->acc.as<double2>() + (((size_t)shot * 3 + comp) * nf) * h->fshot;
     // strip the row padding: [f][nz][ny][px] -> [f][nz][ny][nx]
     CK(cudaMemcpy2DAsync(out, (size_t)h->g.nx * 16, base, (size_t)h->px * 16, (size_t)h->g.nx * 16,
@@ -3010,7 +3023,7 @@ int mittet_stencil_variants(int32_t fp64, int32_t *count, int32_t *cfg, int32_t 
 
 int mittet_time_kernels(mittet_handle *h, int32_t nsteps, double *ms) {
     if (!h || !ms || nsteps <= 0) return fail(MITTET_ERR_INVALID_ARG, "bad timing request");
-    if (h->last_nt < nsteps || h->alloc_shots != h->nshot)
+    if (h->last_nt < nsteps || h->nt_wave < nsteps || h->alloc_shots != h->nshot)
         return fail(MITTET_ERR_STATE, "run a forward of at least %d steps first", nsteps);
     int rc = set_device(h);
     if (rc) return rc;
