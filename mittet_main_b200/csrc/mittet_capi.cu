@@ -908,25 +908,31 @@ int time_graph(mittet_handle *h, cudaGraphExec_t g, float *ms) {
     return MITTET_OK;
 }
 
+// Variables that force a body of the stepped path.
+constexpr const char *kForceStepped[] = {"MITTET_VARIANT", "MITTET_INTERIOR", "MITTET_BOUNDARY", "MITTET_BAND",
+                                         "MITTET_LAYOUT"};
+
 // Chooses between the stepped graph of part kernels and the persistent
 // launch for this grid and batch by timing one captured block of G steps of
-// each, or of all nt steps where they are fewer: the traces and the wavelet
-// end there (MITTET_PERSIST=0 / 1 forces one).  Leaves zero fields behind.
+// each (MITTET_PERSIST=0 / 1 forces one).  Leaves zero fields behind.
 std::mutex g_persist_mu;
-std::map<std::array<long long, 9>, int> g_persist_cache;  // choice per (grid, shots, precision, points, ring, block)
+std::map<std::array<long long, 8>, int> g_persist_cache;  // choice per (grid, shots, precision, points, ring)
 
 template <typename T>
-int decide_persistent(mittet_handle *h, const PhaseArgs<T> &ea, const PhaseArgs<T> &ha, const InjectArgs<T> &ia_m,
-                      const InjectArgs<T> &ia_e, const SampleArgs<T> &sa, int G) {
+int decide_persistent(mittet_handle *h, const PhaseArgs<T> &ea, const PhaseArgs<T> &ha, InjectArgs<T> ia_m,
+                      InjectArgs<T> ia_e, SampleArgs<T> sa, int G) {
     h->persist_decided = true;
     h->persist_vi = -1;
     const char *mode = std::getenv("MITTET_PERSIST");
     const int force = mode ? std::atoi(mode) : -1;
     if (force == 0) return MITTET_OK;
+    // a forced stepped body is what the caller wants to run
+    if (force != 1)
+        for (const char *v : kForceStepped)
+            if (std::getenv(v)) return MITTET_OK;
     CK(h->bar.ensure(sizeof(GridBarrier)));
-    G = std::min(G, sa.nt);
-    const std::array<long long, 9> key = {h->g.nx, h->g.ny, h->g.nz, h->nshot, (long long)h->fp64 + 2 * (force == 1),
-                                          (long long)h->has_mag + 2 * h->has_ele, ea.ring_k, h->nrec, G};
+    const std::array<long long, 8> key = {h->g.nx, h->g.ny, h->g.nz, h->nshot, (long long)h->fp64 + 2 * (force == 1),
+                                          (long long)h->has_mag + 2 * h->has_ele, ea.ring_k, h->nrec};
     if (!std::getenv("MITTET_PERSIST_STALL")) {
         std::lock_guard<std::mutex> lk(g_persist_mu);
         auto it = g_persist_cache.find(key);
@@ -947,6 +953,17 @@ int decide_persistent(mittet_handle *h, const PhaseArgs<T> &ea, const PhaseArgs<
         std::lock_guard<std::mutex> lk(g_persist_mu);
         g_persist_cache[key] = -1;
         return MITTET_OK;
+    }
+    // A solve of fewer steps has neither traces nor a wavelet for the block,
+    // and a shorter block would time the host's launch of the next graph.
+    DevBuf tr, wave;
+    if (sa.nt < G) {
+        CK(tr.ensure((size_t)h->nshot * std::max(h->nrec, 1) * G * sizeof(T)));
+        CK(wave.ensure((size_t)(G + 1) * sizeof(double)));
+        CK(cudaMemsetAsync(wave.p, 0, (size_t)(G + 1) * sizeof(double), h->st));
+        sa.traces = tr.as<T>();
+        sa.nt = G;
+        ia_m.wave = ia_e.wave = wave.as<double>();
     }
     const bool log = std::getenv("MITTET_TUNE_LOG") != nullptr;
     auto capture = [&](int vi, cudaGraphExec_t *out) -> int {
@@ -1043,8 +1060,8 @@ int decide_persistent(mittet_handle *h, const PhaseArgs<T> &ea, const PhaseArgs<
 // it off, as does MITTET_RESIDENT=0.
 template <typename T>
 bool resident_for(mittet_handle *h, int nshot, const mittet_point_source *pts, size_t npts, ResPlan *plan) {
-    for (const char *v : {"MITTET_PERSIST", "MITTET_VARIANT", "MITTET_INTERIOR", "MITTET_BOUNDARY", "MITTET_BAND",
-                          "MITTET_LAYOUT"})
+    if (std::getenv("MITTET_PERSIST")) return false;
+    for (const char *v : kForceStepped)
         if (std::getenv(v)) return false;
     if (const char *v = std::getenv("MITTET_RESIDENT"))
         if (std::atoi(v) == 0) return false;
