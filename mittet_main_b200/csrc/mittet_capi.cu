@@ -943,8 +943,10 @@ int decide_persistent(mittet_handle *h, const PhaseArgs<T> &ea, const PhaseArgs<
         }
     }
     // The persistent launch only competes where a step holds little work
-    // (launch gaps dominate): measured on a B200 it is 1.5x slower than the
-    // stepped graph for one 64^3 shot and 4-6x slower for 32 of them, so it
+    // (launch gaps dominate).  Milliseconds per 128 steps, stepped and best
+    // persistent: 64^3 3.3, 4.0; 8 shots of it 11.7, 23.8; 110^3 5.8, 9.9; FP64
+    // 128x128x96 x 2 shots 24.4, 31.7; 100^3 x 3 25.4, 53.3; it won on 70x44x40 x
+    // 2 shots with both kinds of points and the volume DFT (4.9, 4.3).  So it
     // is timed only for steps of at most 4 M cells (or when forced), and only
     // in the two-cell shapes with short z chunks that came closest.
     const long long step_cells = (long long)h->nshot * h->fshot;

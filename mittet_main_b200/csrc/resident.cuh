@@ -32,11 +32,12 @@
 // wait.  Shots are independent: with
 // G tiles per shot, floor(SMs / G) groups of CTAs each walk their own shots.
 //
-// What bounds it: one pass of a CTA over its vectors takes about 5 us a phase
-// at 64^3 (exchange of flags and rows about 3 us, the rest the issue slots of
-// the general body: about 250 instructions per CPML cell); at 96^3 the body
-// is most of the time (38 Gcell/s; the stepped path's 20 is launch- and
-// L2-bound there).  Tried and slower: halo rows staged by bulk copies (the
+// What bounds it (ncu, 64^3, one pass of a CTA over its vectors, 10.4 us a
+// step): a third of the warps' time goes to the barriers behind the neighbours'
+// flags, and the general body issues 1010 instructions per vector of four cells
+// and phase, 39 % of the issue slots of the 16 warps an SM holds; DRAM is idle.
+// At 96^3 the body is most of the time (38 Gcell/s; the stepped path's 20 is
+// launch- and L2-bound there).  Tried and slower: halo rows staged by bulk copies (the
 // copies wait for the flags, 8 us a phase at 64^3), and 64-bit words that
 // carry data and a message number (every vector polls its own words: 11 us).
 //
