@@ -68,8 +68,11 @@ ResPlan resident_plan(int nx, int ny, int nz, const unsigned char *heavy_y, cons
                 // are heavy along y, z or both) and 0.7 for a full one;
                 // fitted to 4.4 us (32^3 in 64 tiles), 5.3 (64^3, 128 tiles,
                 // one pass), 8.7 (144 tiles, two passes), 13.4 (96^3, three),
-                // 14.0 (64^3 in 36 tiles, four).  Of equal ones fewer tiles
-                // along y (long in y: 5.3 us, long in z: 6.2).
+                // 14.0 (64^3 in 36 tiles, four), all FP32.  An FP64 phase takes
+                // 0.47 to 0.63 of it on 16 tilings (a pass 1.95 us, heavy
+                // rows or not), which ranks tilings by their passes alike.
+                // Of equal ones fewer tiles along y (long in y: 5.3 us, long
+                // in z: 6.2).
                 // without the heavy rows' part already no better: the tile with
                 // the most rows along y and z exists
                 const int nmost = p.ry * p.rz * nvec;
