@@ -9,18 +9,23 @@ namespace mittet {
 
 namespace {
 
-// Threads of a CTA and x cells per thread.  ncu, 128x128x96 with 4 shots and
-// FP64 taus: the cells of the CPML, two thirds of them, take 85 % of the time
-// (1116 warp instructions a vector, 177 bytes of DRAM a cell; the interior 340
-// and 61); there L1 is 51 % busy, DRAM moves 4.0 TB/s, 35 % of the cycles
-// issue, and loads are 71 % of a warp's wait.  Two cells at 80 registers beat
-// four at twice that, as the boxes of a thin CPML are few vectors wide.  6, 7
-// and 8 CTAs an SM (64x64x48; 128x128x96 with 4 and 16 shots; FP64
-// 53x46x41): 22.5, 51.7, 100, 5.7 ms; 23.5, 51.2, 98.8, 5.9; 23.1, 51.4, 99.2,
-// 6.2.  Prefetches, tiles of 8 x 4 x 4 vectors instead of vectors in order,
-// loads of the own field ahead of the taps, and a launch of the interior's own
-// at 64 registers made no step faster.
-constexpr int kNT = 128, kVX = 2, kBlocks = 6;
+// Threads of a CTA and x cells per thread.  ncu, 128x128x96 with 4 shots: 910
+// warp instructions a vector (the mean of all boxes; two thirds of the cells
+// are in the CPML), 39 % of the cycles issue, L1 is half busy, DRAM moves 3.6
+// to 4.5 TB/s, and loads are 69 % of a warp's time.  Two cells at 80 registers
+// beat four at twice that, as the boxes of a thin CPML are few vectors wide.
+// Milliseconds of the adjoint stage (128x128x96 with 16 shots, 60 steps, and 4,
+// 120; 64x64x48 x 4, 256; 108x110x104 x 2, 100; 110x106x108 x 1, 120; FP64
+// 53x46x41 x 2, 150): 96.7, 50.0, 18.0, 15.0, 10.1, 5.7; with 6 CTAs of 128
+// threads, tap offsets from the tables (the tap loads then wait for them), the
+// history through L2 like the rest and both phases in the same order of shots
+// 97.7, 50.8, 18.4, 15.3, 10.5, 5.7.  Over thousands of steps of 16 shots, where
+// the power cap sets the clock, both take 1.72 ms a step.  20, 16 and 12 warps an
+// SM with more registers take 103, 116 and 142 ms of the first; more than 24
+// spill and are no faster.  Prefetches, tiles of 8 x 4 x 4 vectors instead of
+// vectors in order, loads of the own field or the slabs' taus ahead of the taps,
+// and a launch of the interior's own at 64 registers made no step faster.
+constexpr int kNT = 64, kVX = 2, kBlocks = 12;
 
 // Indices into the profile of one axis: sh and b of the own field (H phase:
 // from H, own E).
@@ -44,15 +49,15 @@ __device__ __forceinline__ bool in_axis(const DBox &b, int ax, int v) { return v
 // The y (AX = 1) or z (AX = 2) axis of one vector: adds the transposed
 // differences of the weights to acc.  Along y the from field's z
 // component A goes into the own x and x (X) into z; along z, y into x and x
-// into y.  G: cells general along the axis: coefficients, clamped tap offsets
-// and slab rows come from the axis's table, so that no load waits behind a
-// branch.  GX: lanes may lie outside the update range or the slab.
+// into y.  G: cells general along the axis: coefficients and slab rows come
+// from the axis's table, so that no load waits behind a branch; tap offsets are
+// clamped to the grid.  GX: lanes may lie outside the update range or the slab.
 template <typename T, int VX, bool EPH, int AX, bool G, bool GX>
 __device__ __forceinline__ void adj_axis(const AdjArgs<T> &a, int shot, int i0, int j, int k, const double *__restrict__ A,
                                          const double *__restrict__ X, const double (&ac)[VX], const double (&xc)[VX],
                                          double (&acc)[3][VX]) {
     constexpr int W = EPH ? -1 : -2, C = -W, OTH = 3 - AX, INTO = AX == 1 ? 2 : 1;
-    const int v0 = AX == 1 ? j : k, vo = AX == 1 ? k : j, step = AX == 1 ? a.px : (int)a.plane;
+    const int n = AX == 1 ? a.ny : a.nz, v0 = AX == 1 ? j : k, vo = AX == 1 ? k : j, step = AX == 1 ? a.px : (int)a.plane;
     const DBox &UA = a.fupd[AX == 1 ? 2 : 1], &UX = a.fupd[0];
     const unsigned all = (1u << VX) - 1u;
     const unsigned ma = !in_axis(UA, OTH, vo) ? 0u : GX ? xmask<VX>(i0, UA.lo[0], UA.hi[0]) : all;
@@ -61,9 +66,7 @@ __device__ __forceinline__ void adj_axis(const AdjArgs<T> &a, int shot, int i0, 
     double wa[4][VX], wx[4][VX];
     int l[4];
     double qa[4], qx[4];
-    int d4[4];
     if constexpr (G) {
-        ld4(d4, R->d);
         ld4(l, R->l);
         ld4(qa, R->qa);
         ld4(qx, R->qx);
@@ -72,7 +75,7 @@ __device__ __forceinline__ void adj_axis(const AdjArgs<T> &a, int shot, int i0, 
     for (int t = 0; t < 4; t++) {
         int d = W + t;
         if constexpr (G) {
-            d = d4[t];
+            d = min(max(v0 + d, 0), n - 1) - v0;
         } else {
             qa[t] = a.qk[AX][t];
             qx[t] = -qa[t];
@@ -244,8 +247,8 @@ __device__ __forceinline__ void adj_cells(const AdjArgs<T> &a, int shot, int i0,
         T e0[3][VX], e1[3][VX];
 #pragma unroll
         for (int q = 0; q < 3; q++) {
-            ldv<T, VX>(e0[q], a.S0[q] + sb + c);
-            ldv<T, VX>(e1[q], a.S1[q] + sb + c);
+            ldv_stream<T, VX>(e0[q], a.S0[q] + sb + c);
+            ldv_stream<T, VX>(e1[q], a.S1[q] + sb + c);
         }
         double2 *g = reinterpret_cast<double2 *>(a.grad + sb + c);
 #pragma unroll
@@ -411,7 +414,9 @@ __device__ __forceinline__ void adj_cells(const AdjArgs<T> &a, int shot, int i0,
 }
 
 // All boxes of one phase in one launch, one vector per thread; the body is
-// chosen per CTA.  Corners and edges come first: they take longest.
+// chosen per CTA.  Corners and edges come first: they take longest.  The E
+// phase walks the shots backwards: its first ones are those the H phase left
+// in L2, and the reverse at the next step.
 template <typename T, bool EPH>
 __global__ void __launch_bounds__(kNT, kBlocks)
     adj_phase_kernel(const __grid_constant__ AdjArgs<T> a, const __grid_constant__ AdjBoxes b) {
@@ -424,12 +429,13 @@ __global__ void __launch_bounds__(kNT, kBlocks)
     if (x >= b.vecs[q]) return;
     const int r = x / b.nvx[q], kl = r / b.rows[q];
     const int i0 = b.lo[q][0] + (x - r * b.nvx[q]) * VX, j = b.lo[q][1] + r - kl * b.rows[q], k = b.lo[q][2] + kl;
+    const int shot = EPH ? (int)(gridDim.y - 1u - blockIdx.y) : (int)blockIdx.y;
     switch (b.kind[q]) {
-        case 0: adj_cells<T, VX, EPH, 0>(a, blockIdx.y, i0, j, k); break;
-        case 1: adj_cells<T, VX, EPH, 1>(a, blockIdx.y, i0, j, k); break;
-        case 2: adj_cells<T, VX, EPH, 2>(a, blockIdx.y, i0, j, k); break;
-        case 4: adj_cells<T, VX, EPH, 4>(a, blockIdx.y, i0, j, k); break;
-        default: adj_cells<T, VX, EPH, 7>(a, blockIdx.y, i0, j, k); break;
+        case 0: adj_cells<T, VX, EPH, 0>(a, shot, i0, j, k); break;
+        case 1: adj_cells<T, VX, EPH, 1>(a, shot, i0, j, k); break;
+        case 2: adj_cells<T, VX, EPH, 2>(a, shot, i0, j, k); break;
+        case 4: adj_cells<T, VX, EPH, 4>(a, shot, i0, j, k); break;
+        default: adj_cells<T, VX, EPH, 7>(a, shot, i0, j, k); break;
     }
 }
 

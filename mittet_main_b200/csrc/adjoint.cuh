@@ -25,10 +25,11 @@
 // over 7 seeds on 85x102x80 (5 shots), 64x64x48 (2), 96x80x96 (3) and 64^3
 // (2): 4.3e-7, 2.1e-7, 4.8e-7, 4.8e-7; with FP32 fields 9.6e-7, 3.0e-7,
 // 8.0e-7, 1.1e-6 (stored weights: 8.4e-7, 2.4e-7, 8.4e-7, 1.1e-6).  It costs
-// time on grids that do not fit in L2: adjoint stage of 128x128x96, 16 shots,
-// 60 steps 100 ms (FP32 91, FP64 taus 104, stored weights 86); 4 shots, 120
-// steps 52 (47, 54, 48); 64x64x48, 4 shots, 256 steps 22.5 (21.3, 24.7, 25.8);
-// FP64 53x46x41, 150 steps 5.7 (6.0, 5.7, 9.9).
+// time on grids that do not fit in L2.  Adjoint stage in ms, FP64 fields, FP32
+// fields, FP64 taus too, stored weights: 128x128x96, 16 shots, 60 steps 100, 91,
+// 104, 86; 4 shots, 120 steps 52, 47, 54, 48; 64x64x48, 4 shots, 256 steps 22.5,
+// 21.3, 24.7, 25.8; FP64 53x46x41, 150 steps 5.7 (stored weights 9.9).  Since
+// then adjoint.cu has brought the first column to 96.7, 50.0, 18.0 and 5.7.
 //
 // Adjoint step n (reverse of forward step n):
 //   add the receivers' a_H[n] to B;  H phase (A, tau_E; gradient of the H
@@ -50,13 +51,12 @@ namespace mittet {
 
 // A row of a general axis, for the taps W .. W + 3 around it (W = -2 in the H
 // phase, -1 in the E phase): stencil weight times the curl's sign times 1/kd
-// of the tap, zero outside the update range (qa, qx of the two components the
-// axis carries), stencil weight times c/d (qg, zero outside the slab), the tap
-// offset clamped to the grid and its row in the slab (the sign bit set where
-// it has none).
+// of the tap, zero outside the update range and the grid (qa, qx of the two
+// components the axis carries), stencil weight times c/d (qg, zero outside the
+// slab) and the tap's row in the slab (the sign bit set where it has none).
 struct __align__(16) AdjTapRow {
     double qa[4], qx[4], qg[4];
-    int d[4], l[4];
+    int l[4];
 };
 // Cells along x, one array each (read as vectors, entry 8 is cell 0): signed
 // 1/kd of the z and the y component (zero outside their range), c/d, slab

@@ -1919,7 +1919,6 @@ int adj_tables(mittet_handle *h, bool e, AdjArgs<T> *a) {
                 r.qx[t] = in && u >= ux.lo[ax] && u < ux.hi[ax] ? -k : 0.0;
                 const int l = in ? slab_of(s, u) : -1;
                 r.qg[t] = l >= 0 ? q[t] * prof(ax, CG, u) : 0.0;
-                r.d[t] = c - v;
                 r.l[t] = l >= 0 ? l : (int)0x80000000u;
             }
         }

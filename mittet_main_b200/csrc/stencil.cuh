@@ -118,6 +118,15 @@ __device__ __forceinline__ void stv_stream(T *__restrict__ p, const T (&src)[VX]
     for (int q = 0; q < VX; q++) d[q] = src[q];
     __stcs(reinterpret_cast<V *>(p), v);
 }
+// Streaming load of values that nothing reads again while they are in L2.
+template <typename T, int VX>
+__device__ __forceinline__ void ldv_stream(T (&dst)[VX], const T *__restrict__ p) {
+    using V = typename VecT<T, VX>::type;
+    const V v = __ldcs(reinterpret_cast<const V *>(p));
+    const T *s = reinterpret_cast<const T *>(&v);
+#pragma unroll
+    for (int q = 0; q < VX; q++) dst[q] = s[q];
+}
 template <typename T, int VX>
 __device__ __forceinline__ void zerov(T (&d)[VX]) {
 #pragma unroll
