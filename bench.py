@@ -161,8 +161,11 @@ def run_reference(args, wl):
     threads = os.cpu_count() or 1
     seg = args.ref_seg_steps
     cx, cy, cz = wl.shots[0].points[0][:3]
-    times = O.time_satan_reference(cp.nx, cp.ny, cp.nz, cp.dx, cp.dy, cp.dz, cp.ncpml, cp.omega0, wl.sigma,
-                                   seg, args.warmup + args.steps, (cx, cy, cz), 0, threads)
+    try:
+        times = O.time_satan_reference(cp.nx, cp.ny, cp.nz, cp.dx, cp.dy, cp.dz, cp.ncpml, cp.omega0, wl.sigma,
+                                       seg, args.warmup + args.steps, (cx, cy, cz), 0, threads)
+    except FileNotFoundError:  # compiled where the reference's sources are (oracle/Makefile)
+        return {"impl": "reference", "unavailable": "satan_i's kernels are not built: oracle/_ref/satan_ref_o3 is absent"}
     timed = times[args.warmup:]
     t = float(np.sum(timed))
     ncell = cp.nx * cp.ny * cp.nz
